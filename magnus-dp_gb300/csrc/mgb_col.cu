@@ -39,14 +39,16 @@ bool col_ok(bool plain, int D, int nmax) {
 // long again where FP32 runs wait for it).
 int col_lanes(bool plain, int D, int nmax, int64_t nwork, int64_t kmax, int sms) {
     const int64_t groups = (kmax + 3) / 4, want = (int64_t)sms * (plain ? 64 : 128);
-    const int teams = 32 / D * (plain ? 4 : 2);
+    // A chunk's runs share one CTA, so the geometry that a count selects must hold
+    // that count (d = 3, 4: 32 runs would select 64 threads, 20 or 16 teams).
+    auto fit = [&](int runs) { return runs <= col_geo_t(plain, D, runs, [](auto g) { return g.TC; }); };
     const double group = (4.0 * (nmax - 1) * D * D + 18.0 * nmax * D) * (plain ? 16 : 4);
     const double join = 0.5 * nmax * (nmax - 1) * (D * D + D) * (plain ? 16 : 32);
     // The line: FP32, d = 8, 64 trajectories, n = 4, forward / VJP at 128, 256, 512:
     // 0.21 / 1.09, 0.36 / 1.51, 0.56 / 2.26 ms; FP64 at 64, 128, 256: 3.13 / 8.24,
     // 3.51 / 11.4, 3.03 / 11.9 ms.
     int lpc = 1;
-    while (2 * lpc <= teams && nwork * lpc * D < want && groups >= 4 * lpc &&
+    while (fit(2 * lpc) && nwork * lpc * D < want && groups >= 4 * lpc &&
            groups / (2.0 * lpc) * group > lpc * join)
         lpc *= 2;
     return lpc;

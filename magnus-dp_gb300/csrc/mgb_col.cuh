@@ -617,6 +617,7 @@ cudaError_t col_go(int rule, const LaunchArgs& a, int nmax, bool prepare_only) {
         }
     }
     if (prepare_only) return cudaSuccess;
+    if (a.lpc < 1 || a.lpc > Geo::TC) return cudaErrorInvalidValue;  // a chunk's runs must fit in one CTA
     const int cpb = Geo::TC / a.lpc;
     int64_t blocks = (a.nwork + cpb - 1) / cpb;
     int64_t slot = 0;
