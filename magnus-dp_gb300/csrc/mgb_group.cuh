@@ -53,9 +53,9 @@ __device__ __forceinline__ void group_end(double& base, double&, double s4) { ba
 template <class T>
 struct GroupW {
     T w[4][5];
-    bool per_sample;
+    bool per_sample, riemann;
     __device__ __forceinline__ GroupW(int rule, const RuleCoef<T>& k)
-        : per_sample(rule == R_TRAP || rule == R_RIEMANN) {
+        : per_sample(rule == R_TRAP || rule == R_RIEMANN), riemann(rule == R_RIEMANN) {
 #pragma unroll
         for (int l = 0; l < 4; ++l)
 #pragma unroll
@@ -123,7 +123,24 @@ struct GroupW {
     // group's samples in (local), on the rule's inputs there out; Rb + rlo the
     // cotangent on the anchor from later samples (cy: from beyond the chunk),
     // pend in: on the last input from the later group, out: on the anchor's.
+    // FP32 Trapezoid and Riemann compensate every sample's cotangent, as the
+    // forward pass does its increment: with the group's plain sum the gradient of
+    // 3 x 3 trajectories of nine samples, n = 4, was off by 1.08e-7 (Riemann) and
+    // 9.1e-8 (Trapezoid) instead of 9.6e-8 and 8.2e-8.
     __device__ __forceinline__ void adjoint(T (&v)[4], int cnt, T& Rb, T& rlo, T& pend, bool with_cy, const Carry<T>& cy) const {
+        if (sizeof(T) == 4 && per_sample) {
+#pragma unroll
+            for (int l = 3; l >= 0; --l) {
+                const T h = v[l];
+                if (l >= cnt) continue;
+                acc_add(Rb, rlo, h);
+                T R = Rb + rlo;
+                if (with_cy) R = add_carry(R, cy);
+                v[l] = fma(R, w[0][1], pend);
+                pend = riemann ? T(0) : R * w[0][0];  // (no weight on the anchor: infinities stay out)
+            }
+            return;
+        }
         T H[4];
 #pragma unroll
         for (int l = 0; l < 4; ++l) H[l] = l < cnt ? v[l] : T(0);
