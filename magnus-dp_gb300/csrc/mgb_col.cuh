@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "mgb_common.cuh"
@@ -238,20 +239,24 @@ __global__ void __launch_bounds__(CNT)
                 load_carry(0);
                 for (int j = 0; j < NL; ++j) {
                     const bool emit = emit_top || j + 1 < NL;
+                    auto prefix = [&](auto eachc) {
 #pragma unroll
-                    for (int r = 0; r < D; ++r) {
-                        T base = st(j, 0, r), f0 = st(j, 1, r), lo = F32 ? st(j, NS - 1, r) : T(0);
-                        Carry<T> cy{T(0), T(0)};
-                        if (F32 && carry) cy = Carry<T>{chi[r], clo[r]};
-                        T v[4] = {f[0][r], f[1][r], f[2][r], f[3][r]};
-                        const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
-                        gw.forward(v, cnt, base, lo, f0, F32 && carry, cy, emit);
+                        for (int r = 0; r < D; ++r) {
+                            T base = st(j, 0, r), f0 = st(j, 1, r), lo = F32 ? st(j, NS - 1, r) : T(0);
+                            Carry<T> cy{T(0), T(0)};
+                            if (F32 && carry) cy = Carry<T>{chi[r], clo[r]};
+                            T v[4] = {f[0][r], f[1][r], f[2][r], f[3][r]};
+                            const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
+                            gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, F32 && carry, cy, emit);
 #pragma unroll
-                        for (int l = 0; l < 4; ++l) f[l][r] = v[l];
-                        st(j, 0, r) = base;
-                        if (F32) st(j, NS - 1, r) = lo;
-                        st(j, 1, r) = riem ? T(0) : fl;
-                    }
+                            for (int l = 0; l < 4; ++l) f[l][r] = v[l];
+                            st(j, 0, r) = base;
+                            if (F32) st(j, NS - 1, r) = lo;
+                            st(j, 1, r) = riem ? T(0) : fl;
+                        }
+                    };
+                    if (F32 && gw.each) prefix(std::integral_constant<bool, F32>{});
+                    else prefix(std::false_type{});
                     if (!emit) break;
 #pragma unroll
                     for (int l = 0; l < 4; ++l) {
@@ -513,19 +518,23 @@ __global__ void __launch_bounds__(CNT)
                             }
                             __syncwarp(tmask);
                         }
+                        auto reverse = [&](auto eachc) {
 #pragma unroll
-                        for (int r = 0; r < D; ++r) {
-                            T Rb = st(j, 0, r), pend = st(j, 1, r), rlo = F32 ? st(j, NS - 1, r) : T(0);
-                            Carry<T> cy{T(0), T(0)};
-                            if (F32) cy = Carry<T>{rh[r], rl[r]};
-                            T v[4] = {G[0][r], G[1][r], G[2][r], G[3][r]};
-                            gw.adjoint(v, cnt, Rb, rlo, pend, F32, cy);
+                            for (int r = 0; r < D; ++r) {
+                                T Rb = st(j, 0, r), pend = st(j, 1, r), rlo = F32 ? st(j, NS - 1, r) : T(0);
+                                Carry<T> cy{T(0), T(0)};
+                                if (F32) cy = Carry<T>{rh[r], rl[r]};
+                                T v[4] = {G[0][r], G[1][r], G[2][r], G[3][r]};
+                                gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, F32, cy);
 #pragma unroll
-                            for (int l = 0; l < 4; ++l) G[l][r] = v[l];
-                            st(j, 0, r) = Rb;
-                            st(j, 1, r) = riem ? T(0) : pend;
-                            if (F32) st(j, NS - 1, r) = rlo;
-                        }
+                                for (int l = 0; l < 4; ++l) G[l][r] = v[l];
+                                st(j, 0, r) = Rb;
+                                st(j, 1, r) = riem ? T(0) : pend;
+                                if (F32) st(j, NS - 1, r) = rlo;
+                            }
+                        };
+                        if (F32 && gw.each) reverse(std::integral_constant<bool, F32>{});
+                        else reverse(std::false_type{});
                     }
 #pragma unroll
                     for (int l = 0; l < 4; ++l) {

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "mgb_common.cuh"
@@ -146,20 +147,24 @@ __global__ void __launch_bounds__(256)
                 for (int j = 0; j < NL; ++j) {
                     const bool emit = emit_top || j + 1 < NL;
                     if (mine) {
+                        auto prefix = [&](auto eachc) {
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            T base = st(j, 0, u), f0 = st(j, 1, u), lo = F32 ? st(j, NS - 1, u) : T(0);
-                            Carry<T> cy{T(0), T(0)};
-                            if (F32 && carry && u < nc) cy = Carry<T>{sPI[j * m + r * d + c0 + u], sPI[nm + j * m + r * d + c0 + u]};
-                            T v[4] = {f[0][u], f[1][u], f[2][u], f[3][u]};
-                            const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
-                            gw.forward(v, cnt, base, lo, f0, F32 && carry, cy, emit);
+                            for (int u = 0; u < 4; ++u) {
+                                T base = st(j, 0, u), f0 = st(j, 1, u), lo = F32 ? st(j, NS - 1, u) : T(0);
+                                Carry<T> cy{T(0), T(0)};
+                                if (F32 && carry && u < nc) cy = Carry<T>{sPI[j * m + r * d + c0 + u], sPI[nm + j * m + r * d + c0 + u]};
+                                T v[4] = {f[0][u], f[1][u], f[2][u], f[3][u]};
+                                const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
+                                gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, F32 && carry, cy, emit);
 #pragma unroll
-                            for (int l = 0; l < 4; ++l) f[l][u] = u < nc ? v[l] : T(0);
-                            st(j, 0, u) = base;
-                            if (F32) st(j, NS - 1, u) = lo;
-                            st(j, 1, u) = riem ? T(0) : fl;
-                        }
+                                for (int l = 0; l < 4; ++l) f[l][u] = u < nc ? v[l] : T(0);
+                                st(j, 0, u) = base;
+                                if (F32) st(j, NS - 1, u) = lo;
+                                st(j, 1, u) = riem ? T(0) : fl;
+                            }
+                        };
+                        if (F32 && gw.each) prefix(std::integral_constant<bool, F32>{});
+                        else prefix(std::false_type{});
                         if (emit) {
 #pragma unroll
                             for (int l = 0; l < 4; ++l) {
@@ -297,19 +302,23 @@ __global__ void __launch_bounds__(256)
                     __syncthreads();
                 }
                 if (mine) {
+                    auto reverse = [&](auto eachc) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        T Rb = st(j, 0, u), pend = st(j, 1, u), rlo = F32 ? st(j, NS - 1, u) : T(0);
-                        Carry<T> cy{T(0), T(0)};
-                        if (F32 && u < nc) cy = Carry<T>{sRHO[j * m + r * d + c0 + u], sRHO[nm + j * m + r * d + c0 + u]};
-                        T v[4] = {G[0][u], G[1][u], G[2][u], G[3][u]};
-                        gw.adjoint(v, cnt, Rb, rlo, pend, F32, cy);
+                        for (int u = 0; u < 4; ++u) {
+                            T Rb = st(j, 0, u), pend = st(j, 1, u), rlo = F32 ? st(j, NS - 1, u) : T(0);
+                            Carry<T> cy{T(0), T(0)};
+                            if (F32 && u < nc) cy = Carry<T>{sRHO[j * m + r * d + c0 + u], sRHO[nm + j * m + r * d + c0 + u]};
+                            T v[4] = {G[0][u], G[1][u], G[2][u], G[3][u]};
+                            gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, F32, cy);
 #pragma unroll
-                        for (int l = 0; l < 4; ++l) G[l][u] = u < nc ? v[l] : T(0);
-                        st(j, 0, u) = Rb;
-                        st(j, 1, u) = riem ? T(0) : pend;
-                        if (F32) st(j, NS - 1, u) = rlo;
-                    }
+                            for (int l = 0; l < 4; ++l) G[l][u] = u < nc ? v[l] : T(0);
+                            st(j, 0, u) = Rb;
+                            st(j, 1, u) = riem ? T(0) : pend;
+                            if (F32) st(j, NS - 1, u) = rlo;
+                        }
+                    };
+                    if (F32 && gw.each) reverse(std::integral_constant<bool, F32>{});
+                    else reverse(std::false_type{});
                 }
                 if (n == 1) __syncthreads();
             }
