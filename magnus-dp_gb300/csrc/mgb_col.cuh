@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(CNT)
         const int glast = l1 > l0 ? l0 + 1 + ((l1 - l0 - 1) & ~3) : (riem0 ? 0 : l1 + 1);
 
         // One pass forward over the run: NL levels from the lane's state;
-        // carry: the FP32 start state is added to emitted values, which go to
-        // the tape; emit_top: the last level's values are wanted too
+        // carry: the start state is added to emitted values, which go to the
+        // tape; emit_top: the last level's values are wanted too
         auto forward = [&](int NL, bool carry, bool emit_top) {
             if (g0 > l1 || NL == 0) return;
             int q = 0;
@@ -228,11 +228,11 @@ __global__ void __launch_bounds__(CNT)
                 // a level's carries are asked for ahead of the products before it
                 T chi[D], clo[D];
                 auto load_carry = [&](int j) {
-                    if (F32 && carry) {
+                    if (carry) {
 #pragma unroll
                         for (int r = 0; r < D; ++r) {
                             chi[r] = sPI[j * m + r * D + c];
-                            clo[r] = sPI[nm + j * m + r * D + c];
+                            clo[r] = F32 ? sPI[nm + j * m + r * D + c] : T(0);
                         }
                     }
                 };
@@ -244,10 +244,10 @@ __global__ void __launch_bounds__(CNT)
                         for (int r = 0; r < D; ++r) {
                             T base = st(j, 0, r), f0 = st(j, 1, r), lo = F32 ? st(j, NS - 1, r) : T(0);
                             Carry<T> cy{T(0), T(0)};
-                            if (F32 && carry) cy = Carry<T>{chi[r], clo[r]};
+                            if (carry) cy = Carry<T>{chi[r], clo[r]};
                             T v[4] = {f[0][r], f[1][r], f[2][r], f[3][r]};
                             const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
-                            gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, F32 && carry, cy, emit);
+                            gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, carry, cy, emit);
 #pragma unroll
                             for (int l = 0; l < 4; ++l) f[l][r] = v[l];
                             st(j, 0, r) = base;
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(CNT)
                 }
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
-                    st(j, 0, r) = F32 ? T(0) : sPI[j * m + r * D + c];
+                    st(j, 0, r) = T(0);
                     if (F32) st(j, NS - 1, r) = T(0);
                     st(j, 1, r) = riem ? T(0) : y[r];
                 }
@@ -451,11 +451,11 @@ __global__ void __launch_bounds__(CNT)
             __syncwarp(tmask);
             forward(n - 1, true, true);
 
-            // ---- adjoint: Rb (FP64: from rho), pend, (FP32) rlo
+            // ---- adjoint: Rb, pend, (FP32) rlo
             for (int j = 0; j < n; ++j)
 #pragma unroll
                 for (int r = 0; r < D; ++r) {
-                    st(j, 0, r) = F32 ? T(0) : sRHO[j * m + r * D + c];
+                    st(j, 0, r) = T(0);
                     if (F32) st(j, NS - 1, r) = T(0);
                     st(j, 1, r) = T(0);
                 }
@@ -479,12 +479,10 @@ __global__ void __launch_bounds__(CNT)
                         // products: the carry, and each sample's row of P one
                         // sample early (waiting for them took half of the cycles)
                         T rh[D], rl[D], p[D];
-                        if (F32) {
 #pragma unroll
-                            for (int r = 0; r < D; ++r) {
-                                rh[r] = sRHO[j * m + r * D + c];
-                                rl[r] = sRHO[nm + j * m + r * D + c];
-                            }
+                        for (int r = 0; r < D; ++r) {
+                            rh[r] = sRHO[j * m + r * D + c];
+                            rl[r] = F32 ? sRHO[nm + j * m + r * D + c] : T(0);
                         }
                         const T* const tp = tape + ((int64_t)(li - l0) * (n - 1) + j) * m + c * D;
                         if (j + 1 < n) {
@@ -523,9 +521,9 @@ __global__ void __launch_bounds__(CNT)
                             for (int r = 0; r < D; ++r) {
                                 T Rb = st(j, 0, r), pend = st(j, 1, r), rlo = F32 ? st(j, NS - 1, r) : T(0);
                                 Carry<T> cy{T(0), T(0)};
-                                if (F32) cy = Carry<T>{rh[r], rl[r]};
+                                cy = Carry<T>{rh[r], rl[r]};
                                 T v[4] = {G[0][r], G[1][r], G[2][r], G[3][r]};
-                                gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, F32, cy);
+                                gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, true, cy);
 #pragma unroll
                                 for (int l = 0; l < 4; ++l) G[l][r] = v[l];
                                 st(j, 0, r) = Rb;

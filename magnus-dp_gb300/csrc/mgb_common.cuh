@@ -273,10 +273,8 @@ __device__ __forceinline__ Carry<T> split_carry(double v) {
     c.lo = (T)(v - (double)c.hi);
     return c;
 }
-template <class T>
-__device__ __forceinline__ T add_carry(T local, const Carry<T>& c) {
-    return (local + c.lo) + c.hi;
-}
+__device__ __forceinline__ float add_carry(float local, const Carry<float>& c) { return (local + c.lo) + c.hi; }
+__device__ __forceinline__ double add_carry(double local, const Carry<double>& c) { return local + c.hi; }
 
 // Error-free sum a + b = s + err (Knuth's TwoSum), used to carry the local
 // prefix accumulators at twice the working precision in FP32.

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256)
         const int g0 = riem0 ? 0 : 1, glast = 1 + ((Kp - 1) & ~3);
 
         // forward over the chunk: NL levels; carry: values go to the tape with
-        // the chunk's start state added (FP64: base starts there)
+        // the chunk's start state added
         auto forward = [&](int NL, bool carry, bool emit_top) {
             if (NL == 0) return;
             for (int li = g0; li <= Kp; li = next_of(li)) {
@@ -152,10 +152,13 @@ __global__ void __launch_bounds__(256)
                             for (int u = 0; u < 4; ++u) {
                                 T base = st(j, 0, u), f0 = st(j, 1, u), lo = F32 ? st(j, NS - 1, u) : T(0);
                                 Carry<T> cy{T(0), T(0)};
-                                if (F32 && carry && u < nc) cy = Carry<T>{sPI[j * m + r * d + c0 + u], sPI[nm + j * m + r * d + c0 + u]};
+                                if (carry && u < nc) {
+                                    const int64_t el = (int64_t)j * m + r * d + c0 + u;
+                                    cy = F32 ? Carry<T>{sPI[el], sPI[nm + el]} : Carry<T>{(T)(riem0 ? 0.0 : pic[el]), T(0)};
+                                }
                                 T v[4] = {f[0][u], f[1][u], f[2][u], f[3][u]};
                                 const T fl = cnt == 4 ? v[3] : cnt == 3 ? v[2] : cnt == 2 ? v[1] : v[0];
-                                gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, F32 && carry, cy, emit);
+                                gw.template forward<decltype(eachc)::value>(v, cnt, base, lo, f0, carry, cy, emit);
 #pragma unroll
                                 for (int l = 0; l < 4; ++l) f[l][u] = u < nc ? v[l] : T(0);
                                 st(j, 0, u) = base;
@@ -244,7 +247,7 @@ __global__ void __launch_bounds__(256)
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    st(j, 0, u) = (F32 || riem0 || u >= nc) ? T(0) : (T)pic[(int64_t)j * m + r * d + c0 + u];
+                    st(j, 0, u) = T(0);
                     if (F32) st(j, NS - 1, u) = T(0);
                     st(j, 1, u) = riem ? T(0) : y[u];
                 }
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(256)
             for (int j = 0; j < n; ++j)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    st(j, 0, u) = (F32 || u >= nc) ? T(0) : (T)rcc[(int64_t)j * m + r * d + c0 + u];
+                    st(j, 0, u) = T(0);
                     if (F32) st(j, NS - 1, u) = T(0);
                     st(j, 1, u) = T(0);
                 }
@@ -307,9 +310,12 @@ __global__ void __launch_bounds__(256)
                         for (int u = 0; u < 4; ++u) {
                             T Rb = st(j, 0, u), pend = st(j, 1, u), rlo = F32 ? st(j, NS - 1, u) : T(0);
                             Carry<T> cy{T(0), T(0)};
-                            if (F32 && u < nc) cy = Carry<T>{sRHO[j * m + r * d + c0 + u], sRHO[nm + j * m + r * d + c0 + u]};
+                            if (u < nc) {
+                                const int64_t el = (int64_t)j * m + r * d + c0 + u;
+                                cy = F32 ? Carry<T>{sRHO[el], sRHO[nm + el]} : Carry<T>{(T)rcc[el], T(0)};
+                            }
                             T v[4] = {G[0][u], G[1][u], G[2][u], G[3][u]};
-                            gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, F32, cy);
+                            gw.template adjoint<decltype(eachc)::value>(v, cnt, Rb, rlo, pend, true, cy);
 #pragma unroll
                             for (int l = 0; l < 4; ++l) G[l][u] = u < nc ? v[l] : T(0);
                             st(j, 0, u) = Rb;
