@@ -784,7 +784,7 @@ mgb_status plan_autotune(PlanCore& pc, cudaStream_t st) {
     if (st) cudaStreamIsCapturing(st, &cap);
     for (Segment& sg : pc.segs) {
         const TunedChoice tc0 = choose_tuned(pc.plain, pc.kind, pc.rule, MODE_LOCAL, pc.f64io != 0, sg.hi, 0);
-        const int nv = tc0.use ? (tc0.family == 1 ? 1 : tc0.nvariants) : GENERIC_VARIANTS;
+        const int nv = tc0.use ? (tc0.family == 1 ? 1 : tc0.nvariants) : std::max(tc0.nvariants, GENERIC_VARIANTS);
         if (forced >= 0) {
             sg.variant = forced < nv ? forced : 0;
             continue;

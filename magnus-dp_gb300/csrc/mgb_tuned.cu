@@ -502,6 +502,20 @@ cudaError_t launch_tile(int D, int rule, int mode, const LaunchArgs& a, int grid
                         : launch_tile_m<16, 1>(rule, mode, a, grid, prepare_only);
 }
 
+// Which variant the tile kernel (mgb_dense.cuh) is.  Variant 0 also runs where
+// nothing is timed (mgb_forward_noalloc, MGB_AUTOTUNE=0, inside a capture), so
+// it must be the better one there: FP64, one trajectory of S = 4097, n = 3,
+// forward / forward and VJP, level-major against tiles: d = 12 0.80 / 2.63 against
+// 1.57 / 5.83 ms, d = 15 1.34 / 4.45 against 1.92 / 7.15, d = 20 2.48 / 8.87 against
+// 2.42 / 8.76; mixed d = 9 0.37 / 1.20 against 0.58 / 1.97, d = 12 0.45 / 1.47 against
+// 0.48 / 1.61, d = 13 0.64 / 2.05 against 0.54 / 1.88.  In the mixed form larger
+// calls of d = 9..12 gain from the tiles (d = 12, 32 trajectories, n = 6: 1.65 / 6.15
+// against 0.84 / 4.23): a fourth variant there.  In FP64 none did below 16.
+static int dense_variant(bool plain, int d) {
+    if (plain) return d >= 16 ? 0 : -1;
+    return d >= 13 ? 0 : GENERIC_VARIANTS;
+}
+
 TunedChoice choose_tuned(bool plain, int kind, int rule, int mode, bool f64io, const std::vector<InstDev>& hi,
                          int variant) {
     TunedChoice tc;
@@ -538,12 +552,13 @@ TunedChoice choose_tuned(bool plain, int kind, int rule, int mode, bool f64io, c
         int nm = 0;
         for (const InstDev& I : hi) nm = I.n > nm ? I.n : nm;
         TunedChoice t;
-        if (kind != KIND_MATRIX || variant != 0 || !dense_ok(plain, hi[0].d, nm)) return t;
+        const int at = kind == KIND_MATRIX && dense_ok(plain, hi[0].d, nm) ? dense_variant(plain, hi[0].d) : -1;
+        t.nvariants = at == GENERIC_VARIANTS ? GENERIC_VARIANTS + 1 : GENERIC_VARIANTS;
+        if (variant != at) return t;
         t.use = true;
         t.family = 5;
         t.D = hi[0].d;
         t.nmax = nm;
-        t.nvariants = GENERIC_VARIANTS;
         t.ctas_per_sm = 8;
         return t;
     };

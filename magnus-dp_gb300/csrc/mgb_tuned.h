@@ -70,8 +70,9 @@ int* device_timeout_ptr();
 // One CTA waits (limit_ns) on an mbarrier nothing arrives at and raises the
 // time-out flag (mgb_selftest.cu).
 cudaError_t launch_wait_selftest(uint64_t limit_ns, cudaStream_t st);
-// Generic kernel variants: 8, 4 or 2 CTAs per SM (d = 3..32: the column or
-// tile kernel in place of the first).
+// Generic kernel variants: 8, 4 or 2 CTAs per SM (the column or tile kernel in
+// place of the first, or, for the tile kernel in the mixed form at d = 9..12,
+// after them).
 constexpr int GENERIC_VARIANTS = 3;
 int generic_ctas_per_sm(int variant);
 // 1 if a kernel gave up a bounded device-side wait since the last call.
