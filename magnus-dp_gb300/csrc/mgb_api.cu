@@ -351,9 +351,10 @@ struct Segment {
     bool scan4 = false;     // mixed form, 4-element algebras: double-FP32 scans
     int d = 0, nmax = 0;
     std::vector<int32_t> active;
-    // chunk-kernel launch variant (autotuner) and the times it measured
-    int variant = 0;
-    std::vector<float> tune_ms;
+    // chunk-kernel launch variants (autotuner) of the forward local pass and of
+    // the VJP, and the times it measured
+    int variant = 0, vjp_variant = 0;
+    std::vector<float> tune_ms, vjp_ms;
     bool tuned_here = false;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
@@ -716,7 +717,8 @@ mgb_status plan_upload(PlanCore& pc, cudaStream_t st, bool synchronous) {
 mgb_status plan_streams(PlanCore& pc) {
     for (const Segment& sg : pc.segs) {
         for (int mode : {MODE_LOCAL, MODE_VJP})
-            MGB_CUDA_TRY(prepare_tuned(choose_tuned(pc.plain, pc.kind, pc.rule, mode, pc.f64io != 0, sg.hi, sg.variant),
+            MGB_CUDA_TRY(prepare_tuned(choose_tuned(pc.plain, pc.kind, pc.rule, mode, pc.f64io != 0, sg.hi,
+                                                    mode == MODE_VJP ? sg.vjp_variant : sg.variant),
                                        pc.rule, mode));
         if (sg.df_scan)
             for (bool rev : {false, true})
@@ -749,20 +751,27 @@ LaunchArgs seg_args(const PlanCore& pc, const Segment& sg, cudaStream_t st) {
 // ---------------------------------------------------------------- autotuner
 // Each chunk-kernel family has launch variants (mgb_tuned.h): k-block and CTAs
 // per SM of the tensor-core kernel, CTAs per SM (register budget) of the
-// group-tiled kernel, CTAs per SM of the generic kernel.  Before a plan's
-// first use, every variant of each segment's kernel runs the forward local
-// pass over a sample of the segment's chunks (two waves of resident CTAs,
-// spread over its instances, chunk totals written to a private buffer so no
-// caller buffer is touched) and the fastest is kept.  Results are cached for
-// the process by (family, d, rule, order bound, form, teams per chunk).  MGB_AUTOTUNE=0 turns
-// tuning off (variant 0 everywhere); MGB_FORCE_VARIANT=k forces variant k
-// (tests use it to check every variant against the oracle).
+// group-tiled kernel, CTAs per SM of the generic kernel, and at d = 3..32 the
+// column or tile kernel beside it.  Before a plan's first use, every variant of
+// each segment's kernel runs the forward local pass over a sample of the
+// segment's chunks (two waves of resident CTAs, spread over its instances,
+// chunk totals written to a private buffer so no caller buffer is touched)
+// and the fastest is kept.  Where the variants are different kernels (d = 3..32)
+// the VJP has its own pick, timed the same way with a private dA: one FP64
+// trajectory of d = 8, S = 4097, n = 6 had run its VJP at 3.0 ms on the forward
+// pass's pick, against 2.2.  Results are cached for the process by (pass,
+// family, d, rule, order bound, form, teams per chunk, and the load: chunks per
+// SM below 1, up to 8 or above, and the longest chunk to a power of two), so
+// that what a call of a few chunks measured does not decide for a full one
+// (d = 16 FP64, 32 trajectories after a single one: 11.2 ms on the level-major
+// kernel that suited the single one, 8.5 on the tile kernel).  MGB_AUTOTUNE=0
+// turns tuning off (variant 0 everywhere); MGB_FORCE_VARIANT=k forces variant
+// k (tests use it to check every variant against the oracle).
 struct TuneKey {
-    int family, D, rule, nmax, plain, kind, f64io, lpc;
-    bool operator<(const TuneKey& o) const {
-        return std::tie(family, D, rule, nmax, plain, kind, f64io, lpc) <
-               std::tie(o.family, o.D, o.rule, o.nmax, o.plain, o.kind, o.f64io, o.lpc);
-    }
+    int mode, family, D, rule, nmax, plain, kind, f64io, lpc, load, len;
+    auto all() const { return std::tie(mode, family, D, rule, nmax, plain, kind, f64io, lpc, load, len); }
+    auto but_load() const { return std::tie(mode, family, D, rule, nmax, plain, kind, f64io); }
+    bool operator<(const TuneKey& o) const { return all() < o.all(); }
 };
 struct TuneResult {
     int variant = 0;
@@ -777,6 +786,94 @@ int env_int(const char* name, int dflt) {
     return std::atoi(v);
 }
 
+// Times the nv variants of one pass (MODE_LOCAL or MODE_VJP) of a segment's
+// chunk kernel; *ms stays empty where there is no room to.
+mgb_status tune_pass(PlanCore& pc, Segment& sg, int mode, const TunedChoice& tc0, int nv, cudaStream_t st,
+                     std::vector<float>* out) {
+    const bool vjp = mode == MODE_VJP;
+    // sample: up to two waves of the most resident CTAs, round-robin over
+    // the segment's instances, chunk indices below csub per instance
+    // (the column kernel runs several chunks per CTA)
+    const int maxctas = !tc0.use || tc0.family == 5 ? 8 : tc0.family == 4 ? 16 : std::max(tc0.ctas_per_sm, 2);
+    const int64_t target = std::min<int64_t>(sg.nwork, 2LL * pc.sms * maxctas);
+    const int nsub = (int)std::min<int64_t>(sg.count, target);
+    int csub = (int)((target + nsub - 1) / nsub);
+    std::vector<InstDev> sub(pc.hi.begin() + sg.first, pc.hi.begin() + sg.first + nsub);
+    int64_t kmax = 1, nm = 1, m = sub[0].m;
+    for (const InstDev& I : sub) {
+        kmax = std::max<int64_t>(kmax, I.K);
+        nm = std::max<int64_t>(nm, (int64_t)I.n * I.m);
+    }
+    const int64_t es = pc.f64io ? 8 : 4;
+    // VJP: one dA for all sampled instances (its values are not looked at), at
+    // most 256 MB of it, and carries of zero
+    if (vjp) csub = (int)std::max<int64_t>(1, std::min<int64_t>(csub, ((int64_t)256 << 20) / (kmax * m * es)));
+    std::vector<ChunkRef> work;
+    size_t lam_doubles = 0;
+    std::vector<size_t> lam_off(nsub);
+    for (int k = 0; k < nsub; ++k) {
+        lam_off[k] = lam_doubles;
+        if (!vjp) lam_doubles += (size_t)std::min(csub, sub[k].C) * (size_t)sub[k].n * (size_t)sub[k].m;
+    }
+    for (int c = 0; c < csub && (int64_t)work.size() < target; ++c)
+        for (int k = 0; k < nsub && (int64_t)work.size() < target; ++k)
+            if (c < sub[k].C) work.push_back(ChunkRef{k, c});
+    char* tmp = nullptr;
+    const size_t b_inst = align_up(sub.size() * sizeof(InstDev), 256);
+    const size_t b_work = align_up(work.size() * sizeof(ChunkRef), 256);
+    const size_t b_lam = align_up(lam_doubles * sizeof(double), 256);
+    const size_t b_pi = vjp ? align_up((size_t)(csub + 1) * (size_t)nm * sizeof(double), 256) : 0;
+    const size_t b_dA = vjp ? ((size_t)csub * (size_t)kmax + 1) * (size_t)m * (size_t)es : 0;
+    const size_t bytes = b_inst + b_work + b_lam + 2 * b_pi + b_dA;
+    if (cudaMalloc(&tmp, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return MGB_OK;  // no room to tune
+    }
+    char* const tail = tmp + b_inst + b_work;
+    for (int k = 0; k < nsub; ++k) {
+        if (vjp) {
+            sub[k].pi = reinterpret_cast<double*>(tail);
+            sub[k].rho = reinterpret_cast<double*>(tail + b_pi);
+            sub[k].dA = tail + 2 * b_pi;
+        } else {
+            sub[k].lam = reinterpret_cast<double*>(tail) + lam_off[k];
+        }
+    }
+    cudaError_t e = cudaMemcpy(tmp, sub.data(), sub.size() * sizeof(InstDev), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(tmp + b_inst, work.data(), work.size() * sizeof(ChunkRef), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && vjp) e = cudaMemsetAsync(tail, 0, 2 * b_pi, st);
+    LaunchArgs la = seg_args(pc, sg, st);
+    la.insts = reinterpret_cast<const InstDev*>(tmp);
+    la.work = reinterpret_cast<const ChunkRef*>(tmp + b_inst);
+    la.nwork = (int64_t)work.size();
+    std::vector<float> ms(nv, -1.f);
+    const int reps = vjp ? 1 : 2;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (e == cudaSuccess) e = cudaEventCreate(&e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&e1);
+    for (int v = 0; v < nv && e == cudaSuccess; ++v) {
+        cudaError_t r = launch_chunk_any(pc.plain, pc.kind, pc.rule, mode, la, sg.hi, pc.sms, v);  // warm-up
+        if (r == cudaSuccess) r = cudaEventRecord(e0, st);
+        for (int rep = 0; rep < reps && r == cudaSuccess; ++rep)
+            r = launch_chunk_any(pc.plain, pc.kind, pc.rule, mode, la, sg.hi, pc.sms, v);
+        if (r == cudaSuccess) r = cudaEventRecord(e1, st);
+        if (r == cudaSuccess) r = cudaEventSynchronize(e1);
+        float t = 0.f;
+        if (r == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) ms[v] = t / (float)reps;
+        else cudaGetLastError();
+        if (r != cudaSuccess && r != cudaErrorInvalidValue && r != cudaErrorInvalidConfiguration &&
+            r != cudaErrorLaunchOutOfResources)
+            e = r;  // a sticky error: stop
+    }
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    cudaFree(tmp);
+    if (e != cudaSuccess) return fail(MGB_ERR_CUDA, std::string("autotune: ") + cudaGetErrorString(e));
+    if (read_clear_device_timeout()) return fail(MGB_ERR_DEVICE_TIMEOUT, "autotune: a device-side wait timed out");
+    *out = std::move(ms);
+    return MGB_OK;
+}
+
 mgb_status plan_autotune(PlanCore& pc, cudaStream_t st) {
     const int forced = env_int("MGB_FORCE_VARIANT", -1);
     const bool enabled = env_int("MGB_AUTOTUNE", 1) != 0;
@@ -786,86 +883,48 @@ mgb_status plan_autotune(PlanCore& pc, cudaStream_t st) {
         const TunedChoice tc0 = choose_tuned(pc.plain, pc.kind, pc.rule, MODE_LOCAL, pc.f64io != 0, sg.hi, 0);
         const int nv = tc0.use ? (tc0.family == 1 ? 1 : tc0.nvariants) : std::max(tc0.nvariants, GENERIC_VARIANTS);
         if (forced >= 0) {
-            sg.variant = forced < nv ? forced : 0;
+            sg.variant = sg.vjp_variant = forced < nv ? forced : 0;
             continue;
         }
         if (nv <= 1 || !enabled) continue;
-        const TuneKey key{tc0.use ? tc0.family : 0, sg.d, pc.rule, sg.nmax, pc.plain ? 1 : 0, pc.kind, pc.f64io, sg.lpc};
-        {
-            std::lock_guard<std::mutex> lock(g_tune_mu);
-            auto it = g_tune.find(key);
-            if (it != g_tune.end()) {
-                sg.variant = it->second.variant;
-                sg.tune_ms = it->second.ms;
-                continue;
+        const int load = sg.nwork < pc.sms ? 0 : sg.nwork <= 8LL * pc.sms ? 1 : 2;
+        int len = 0;
+        while (((int64_t)1 << len) < sg.kmax) ++len;
+        auto pick = [&](int mode, int& variant, std::vector<float>& times) -> mgb_status {
+            const TuneKey key{mode, tc0.use ? tc0.family : 0, sg.d, pc.rule, sg.nmax, pc.plain ? 1 : 0, pc.kind, pc.f64io,
+                              sg.lpc, load, len};
+            const bool capturing = cap != cudaStreamCaptureStatusNone;  // no timing inside a capture
+            {
+                std::lock_guard<std::mutex> lock(g_tune_mu);
+                auto it = g_tune.find(key);
+                // (there, another load's pick rather than none)
+                if (it == g_tune.end() && capturing)
+                    it = std::find_if(g_tune.begin(), g_tune.end(), [&](const auto& x) { return x.first.but_load() == key.but_load(); });
+                if (it != g_tune.end()) {
+                    variant = it->second.variant;
+                    times = it->second.ms;
+                    return MGB_OK;
+                }
             }
-        }
-        if (cap != cudaStreamCaptureStatusNone) continue;  // no timing inside a capture
-        // sample: up to two waves of the most resident CTAs, round-robin over
-        // the segment's instances, chunk indices below csub per instance
-        // (the column kernel runs several chunks per CTA)
-        const int maxctas = !tc0.use || tc0.family == 5 ? 8 : tc0.family == 4 ? 16 : std::max(tc0.ctas_per_sm, 2);
-        const int64_t target = std::min<int64_t>(sg.nwork, 2LL * pc.sms * maxctas);
-        const int nsub = (int)std::min<int64_t>(sg.count, target);
-        const int csub = (int)((target + nsub - 1) / nsub);
-        std::vector<InstDev> sub(pc.hi.begin() + sg.first, pc.hi.begin() + sg.first + nsub);
-        std::vector<ChunkRef> work;
-        size_t lam_doubles = 0;
-        std::vector<size_t> lam_off(nsub);
-        for (int k = 0; k < nsub; ++k) {
-            lam_off[k] = lam_doubles;
-            lam_doubles += (size_t)std::min(csub, sub[k].C) * (size_t)sub[k].n * (size_t)sub[k].m;
-        }
-        for (int c = 0; c < csub && (int64_t)work.size() < target; ++c)
-            for (int k = 0; k < nsub && (int64_t)work.size() < target; ++k)
-                if (c < sub[k].C) work.push_back(ChunkRef{k, c});
-        char* tmp = nullptr;
-        const size_t b_inst = align_up(sub.size() * sizeof(InstDev), 256);
-        const size_t b_work = align_up(work.size() * sizeof(ChunkRef), 256);
-        const size_t bytes = b_inst + b_work + lam_doubles * sizeof(double);
-        if (cudaMalloc(&tmp, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            continue;  // no room to tune: keep variant 0
-        }
-        double* lam = reinterpret_cast<double*>(tmp + b_inst + b_work);
-        for (int k = 0; k < nsub; ++k) sub[k].lam = lam + lam_off[k];
-        cudaError_t e = cudaMemcpy(tmp, sub.data(), sub.size() * sizeof(InstDev), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(tmp + b_inst, work.data(), work.size() * sizeof(ChunkRef), cudaMemcpyHostToDevice);
-        LaunchArgs la = seg_args(pc, sg, st);
-        la.insts = reinterpret_cast<const InstDev*>(tmp);
-        la.work = reinterpret_cast<const ChunkRef*>(tmp + b_inst);
-        la.nwork = (int64_t)work.size();
-        std::vector<float> ms(nv, -1.f);
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        if (e == cudaSuccess) e = cudaEventCreate(&e0);
-        if (e == cudaSuccess) e = cudaEventCreate(&e1);
-        for (int v = 0; v < nv && e == cudaSuccess; ++v) {
-            cudaError_t r = launch_chunk_any(pc.plain, pc.kind, pc.rule, MODE_LOCAL, la, sg.hi, pc.sms, v);  // warm-up
-            if (r == cudaSuccess) r = cudaEventRecord(e0, st);
-            for (int rep = 0; rep < 2 && r == cudaSuccess; ++rep)
-                r = launch_chunk_any(pc.plain, pc.kind, pc.rule, MODE_LOCAL, la, sg.hi, pc.sms, v);
-            if (r == cudaSuccess) r = cudaEventRecord(e1, st);
-            if (r == cudaSuccess) r = cudaEventSynchronize(e1);
-            float t = 0.f;
-            if (r == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) ms[v] = t / 2.f;
-            else cudaGetLastError();
-            if (r != cudaSuccess && r != cudaErrorInvalidValue && r != cudaErrorInvalidConfiguration &&
-                r != cudaErrorLaunchOutOfResources)
-                e = r;  // a sticky error: stop
-        }
-        if (e0) cudaEventDestroy(e0);
-        if (e1) cudaEventDestroy(e1);
-        cudaFree(tmp);
-        if (e != cudaSuccess) return fail(MGB_ERR_CUDA, std::string("autotune: ") + cudaGetErrorString(e));
-        if (read_clear_device_timeout()) return fail(MGB_ERR_DEVICE_TIMEOUT, "autotune: a device-side wait timed out");
-        int best = 0;
-        for (int v = 0; v < nv; ++v)
-            if (ms[v] >= 0.f && (ms[best] < 0.f || ms[v] < ms[best])) best = v;
-        sg.variant = best;
-        sg.tune_ms = ms;
-        sg.tuned_here = true;
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        g_tune[key] = TuneResult{best, ms};
+            if (capturing) return MGB_OK;
+            std::vector<float> ms;
+            mgb_status s = tune_pass(pc, sg, mode, tc0, nv, st, &ms);
+            if (s != MGB_OK || ms.empty()) return s;
+            int best = 0;
+            for (int v = 0; v < nv; ++v)
+                if (ms[v] >= 0.f && (ms[best] < 0.f || ms[v] < ms[best])) best = v;
+            variant = best;
+            times = ms;
+            sg.tuned_here = true;
+            std::lock_guard<std::mutex> lock(g_tune_mu);
+            g_tune[key] = TuneResult{best, ms};
+            return MGB_OK;
+        };
+        mgb_status s = pick(MODE_LOCAL, sg.variant, sg.tune_ms);
+        sg.vjp_variant = sg.variant;
+        const bool kernels = tc0.use ? tc0.family >= 4 : nv > GENERIC_VARIANTS;  // the variants are different kernels
+        if (s == MGB_OK && pc.has_vjp && kernels) s = pick(MODE_VJP, sg.vjp_variant, sg.vjp_ms);
+        if (s != MGB_OK) return s;
     }
     return MGB_OK;
 }
@@ -888,7 +947,8 @@ mgb_status for_segments(PlanCore& pc, cudaStream_t st, F&& f) {
 
 mgb_status seg_chunks(PlanCore& pc, Segment& sg, int mode, cudaStream_t s, const char* name) {
     const LaunchArgs la = seg_args(pc, sg, s);
-    MGB_CUDA_TRY(timed(name, s, [&] { return launch_chunk_any(pc.plain, pc.kind, pc.rule, mode, la, sg.hi, pc.sms, sg.variant); }));
+    MGB_CUDA_TRY(timed(name, s, [&] { return launch_chunk_any(pc.plain, pc.kind, pc.rule, mode, la, sg.hi, pc.sms,
+                                                         mode == MODE_VJP ? sg.vjp_variant : sg.variant); }));
     return MGB_OK;
 }
 
@@ -1262,10 +1322,16 @@ size_t mgb_plan_describe(const mgb_plan* plan, char* buf, size_t len) {
                       i ? ", " : "", sg.d, sg.count, (long long)sg.nwork, kernel, sg.variant, ctas, (long long)sg.grid,
                       sg.tiled_scan ? "tiled" : "per-instance");
         o += tmp;
-        for (size_t v = 0; v < sg.tune_ms.size(); ++v) {
-            std::snprintf(tmp, sizeof(tmp), "%s%.9g", v ? ", " : "", (double)sg.tune_ms[v]);
-            o += tmp;
-        }
+        auto list = [&](const std::vector<float>& ms) {
+            for (size_t v = 0; v < ms.size(); ++v) {
+                std::snprintf(tmp, sizeof(tmp), "%s%.9g", v ? ", " : "", (double)ms[v]);
+                o += tmp;
+            }
+        };
+        list(sg.tune_ms);
+        std::snprintf(tmp, sizeof(tmp), "], \"vjp_variant\": %d, \"vjp_ms\": [", sg.vjp_variant);
+        o += tmp;
+        list(sg.vjp_ms);
         o += "]}";
     }
     o += "]}";
