@@ -671,16 +671,25 @@ void keep_upload(std::vector<char>&& src, cudaEvent_t done) {
         std::lock_guard<std::mutex> lock(g_upload_mutex);
         for (auto it = g_uploads.begin(); it != g_uploads.end();) {
             auto next = std::next(it);
-            if (cudaEventQuery(it->done) != cudaErrorNotReady) over.splice(over.end(), g_uploads, it);
+            // a source goes only when its copy is known to be done (a query that
+            // fails, as beside another thread's capture, says nothing)
+            if (cudaEventQuery(it->done) == cudaSuccess) over.splice(over.end(), g_uploads, it);
             else cudaGetLastError();  // not an error: keep it from the next launch's check
             it = next;
         }
         if (g_uploads.size() >= kUploads) over.splice(over.end(), g_uploads, g_uploads.begin());
         g_uploads.push_back(Upload{std::move(src), done});
     }
-    for (Upload& u : over) {  // outside the lock: the oldest may still have to be waited for
-        cudaEventSynchronize(u.done);
-        cudaEventDestroy(u.done);
+    for (auto it = over.begin(); it != over.end();) {  // outside the lock: the oldest may still have to be waited for
+        auto next = std::next(it);
+        if (cudaEventSynchronize(it->done) == cudaSuccess) {
+            cudaEventDestroy(it->done);
+        } else {
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lock(g_upload_mutex);
+            g_uploads.splice(g_uploads.begin(), over, it);
+        }
+        it = next;
     }
 }
 
