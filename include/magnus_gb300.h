@@ -184,6 +184,12 @@ mgb_status mgb_forward_noalloc(const mgb_problem* p, const void* A, void* out, v
 mgb_status mgb_set_gl_table(size_t max_order, const double* weights, const double* nodes);
 size_t mgb_max_order(void);
 
+/* Engine-specific, no reference counterpart.  The one-shot entry points keep up
+ * to 1 GiB of freed workspace per device for their next calls.  This
+ * synchronizes the current device and gives it back, for a program whose other
+ * allocators need the memory. */
+mgb_status mgb_release_workspaces(void);
+
 /* Engine-specific, no reference counterpart.  Synchronizes the current
  * device and returns MGB_ERR_DEVICE_TIMEOUT if a kernel gave up one of its
  * bounded device-side waits since the last check (its outputs are then

@@ -230,7 +230,7 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // everything back at each synchronisation, so that every call mapped its
 // workspace anew (d = 16, 64 trajectories: 0.8 GB).  Memory above the line is
 // given back at the next synchronisation, and all of it when an allocation of
-// this library fails (trim_workspaces).
+// this library fails or the program asks for it (mgb_release_workspaces).
 constexpr uint64_t kPoolKeep = (uint64_t)1 << 30;
 std::mutex g_pool_mutex;
 std::vector<std::pair<cudaMemPool_t, bool>> g_pools;  // per device: pool, looked up
@@ -279,7 +279,7 @@ cudaError_t device_alloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        trim_workspaces();
+        if (cudaDeviceSynchronize() == cudaSuccess) trim_workspaces();  // (blocks still in use stay)
         e = cudaMalloc(p, bytes);
     }
     return e;
@@ -834,7 +834,7 @@ mgb_status tune_pass(PlanCore& pc, Segment& sg, int mode, const TunedChoice& tc0
     const size_t b_pi = vjp ? align_up((size_t)(csub + 1) * (size_t)nm * sizeof(double), 256) : 0;
     const size_t b_dA = vjp ? ((size_t)csub * (size_t)kmax + 1) * (size_t)m * (size_t)es : 0;
     const size_t bytes = b_inst + b_work + b_lam + 2 * b_pi + b_dA;
-    if (cudaMalloc(&tmp, bytes) != cudaSuccess) {
+    if (device_alloc(reinterpret_cast<void**>(&tmp), bytes) != cudaSuccess) {
         cudaGetLastError();
         return MGB_OK;  // no room to tune
     }
@@ -1350,6 +1350,13 @@ size_t mgb_plan_describe(const mgb_plan* plan, char* buf, size_t len) {
         buf[n] = 0;
     }
     return o.size() + 1;
+}
+
+mgb_status mgb_release_workspaces(void) {
+    g_last_error.clear();
+    MGB_CUDA_TRY(cudaDeviceSynchronize());
+    trim_workspaces();
+    return MGB_OK;
 }
 
 mgb_status mgb_plan_destroy(mgb_plan* plan) {

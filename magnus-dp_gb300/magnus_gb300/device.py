@@ -13,6 +13,7 @@ from typing import Callable
 
 import torch
 
+from . import _lib
 from .autograd import magnus, magnus_sc
 
 
@@ -42,3 +43,10 @@ def expm(omega):
     """Matrix exponential of Omega (..., d, d) on its device (the consumer of
     a Magnus sum: the propagator exp(Omega)); batched, differentiable."""
     return torch.linalg.matrix_exp(omega)
+
+
+def release_workspaces():
+    """Give back the workspace memory that one-shot calls keep on the current
+    device for the next ones (at most 1 GiB), after synchronising it: torch's
+    allocator cannot reclaim it by itself."""
+    _lib.check(_lib.load().mgb_release_workspaces())
