@@ -302,7 +302,7 @@ def _plan(lib, _lib, probs, A, out, cot=None, dA=None):
 
 
 def _describe(lib, plan):
-    """The plan's segments: chunk kernel, the launch variant the autotuner
+    """The plan's segments: chunk kernels, the launch variants the autotuner
     picked and the per-variant times it measured."""
     import ctypes as ct
     need = lib.mgb_plan_describe(plan, None, 0)
@@ -529,7 +529,7 @@ def run_config3(args):
                                  n=n, samples=S, dim=d, t0=0.0, tf=1.0)
         return A, cot, prob
 
-    picks = {}  # autotuner picks over the timed waves: "d<d> <kernel> v<variant>" -> segments
+    picks = {}  # autotuner picks over the timed waves: "d<d> <forward kernel> v<variant> <VJP kernel> v<variant>" -> segments
 
     def run_wave(idx, prec, steps, record=False):
         As, cots, probs = [], [], []
@@ -548,7 +548,7 @@ def run_config3(args):
         ms = _time_graph(torch, step, steps, warmup=1)
         if record:
             for sg in _describe(lib, plan):
-                key = f"d{sg['d']} {sg['kernel']} v{sg['variant']}"
+                key = f"d{sg['d']} {sg['forward']} v{sg['variant']} {sg['vjp']} v{sg['vjp_variant']}"
                 picks[key] = picks.get(key, 0) + 1
         lib.mgb_plan_destroy(plan)
         del As, dAs, outs

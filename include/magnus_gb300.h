@@ -128,9 +128,12 @@ mgb_status mgb_plan_forward(mgb_plan* plan, void* stream);
 mgb_status mgb_plan_vjp(mgb_plan* plan, void* stream);
 size_t mgb_plan_bytes(const mgb_plan* plan);
 /* Engine-specific, no reference counterpart: a JSON description of the plan's
- * segments (dimension, instances, chunks, chunk kernel, the launch variant the
- * autotuner chose and the per-variant times it measured in ms, scan kind)
- * written to buf (truncated to len - 1 bytes, NUL-terminated); returns the
+ * segments: d, instances, chunks; kernel (the family whose variants are
+ * counted), forward and vjp (the chunk kernels that run), variant and tuned_ms,
+ * vjp_variant and vjp_ms (the launch variants the autotuner chose and the
+ * per-variant times it measured in ms; vjp_ms is empty where the VJP follows
+ * the forward pass), ctas_per_sm of the forward kernel (0: as many as the
+ * chunks ask for), slots, scan (tiled, columns or per-instance).  Written to buf (truncated to len - 1 bytes, NUL-terminated); returns the
  * length needed including the NUL. */
 size_t mgb_plan_describe(const mgb_plan* plan, char* buf, size_t len);
 mgb_status mgb_plan_destroy(mgb_plan* plan);

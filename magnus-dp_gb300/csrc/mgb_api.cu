@@ -1315,21 +1315,23 @@ size_t mgb_plan_describe(const mgb_plan* plan, char* buf, size_t len) {
     if (!plan) return 0;
     const PlanCore& pc = plan->pc;
     std::string o = "{\"segments\": [";
-    char tmp[256];
+    char tmp[512];
     for (size_t i = 0; i < pc.segs.size(); ++i) {
         const Segment& sg = pc.segs[i];
         const TunedChoice tc = choose_tuned(pc.plain, pc.kind, pc.rule, MODE_LOCAL, pc.f64io != 0, sg.hi, sg.variant);
-        // the forward local pass's kernel; at d = 32 variants 2 and 3 run the
-        // VJP on the warp-MMA kernel
+        const TunedChoice tv = choose_tuned(pc.plain, pc.kind, pc.rule, MODE_VJP, pc.f64io != 0, sg.hi, sg.vjp_variant);
+        // "kernel": the family whose variants are counted
         const char* kernel = !tc.use || tc.family >= 4 ? "k_chunk" : tc.family == 1 ? "k_small" : tc.family == 3 ? "k_bigtc"
                              : (tc.D == 32 && sg.variant == 2) ? "k_tiletc"
                              : (tc.D == 32 && sg.variant == 3) ? "k_mma32" : "k_tile";
-        const int ctas = !tc.use || tc.family >= 4 ? generic_ctas_per_sm(sg.variant % GENERIC_VARIANTS) : tc.ctas_per_sm;
+        const bool curve = tc.use && tc.family == 1 && pc.kind == KIND_SC && !pc.plain && !pc.f64io && sg.lpc == 1;
         std::snprintf(tmp, sizeof(tmp),
-                      "%s{\"d\": %d, \"instances\": %d, \"chunks\": %lld, \"kernel\": \"%s\", \"variant\": %d, "
-                      "\"ctas_per_sm\": %d, \"slots\": %lld, \"scan\": \"%s\", \"tuned_ms\": [",
-                      i ? ", " : "", sg.d, sg.count, (long long)sg.nwork, kernel, sg.variant, ctas, (long long)sg.grid,
-                      sg.tiled_scan ? "tiled" : "per-instance");
+                      "%s{\"d\": %d, \"instances\": %d, \"chunks\": %lld, \"kernel\": \"%s\", \"forward\": \"%s\", "
+                      "\"vjp\": \"%s\", \"variant\": %d, \"ctas_per_sm\": %d, \"slots\": %lld, \"scan\": \"%s\", \"tuned_ms\": [",
+                      i ? ", " : "", sg.d, sg.count, (long long)sg.nwork, kernel,
+                      curve ? "k_curve_local" : kernel_name(tc, MODE_LOCAL), kernel_name(tv, MODE_VJP), sg.variant,
+                      kernel_ctas_per_sm(tc, sg.variant, MODE_LOCAL), (long long)sg.grid,
+                      sg.df_scan ? (scan_by_columns(sg.nmax) ? "columns" : "per-instance") : sg.tiled_scan ? "tiled" : "per-instance");
         o += tmp;
         auto list = [&](const std::vector<float>& ms) {
             for (size_t v = 0; v < ms.size(); ++v) {

@@ -68,6 +68,7 @@ bool scan_tiled_ok(int kind, int d);
 // stored as FP32 pairs (InstDev::lam_pair).
 bool scan_pair_dim(int kind, int d);
 bool scan_df_ok(int kind, int d, int nmax);
+bool scan_by_columns(int nmax);  // (of these) a block of columns per CTA, not an instance
 cudaError_t launch_scan_df(const InstDev* insts, int count, int d, int nmax, bool reverse, int f64io,
                            cudaStream_t st, bool prepare_only = false);
 // The same for the 4-element algebras at orders up to 8 (transfers in FP64).

@@ -604,6 +604,24 @@ static bool forward_cmma(const TunedChoice& tc, int mode) {
     return mode == MODE_LOCAL && ((tc.family == 2 && tc.D == 32 && tc.variant == 3) || (tc.family == 3 && tc.D == 64 && tc.variant == 2));
 }
 
+const char* kernel_name(const TunedChoice& tc, int mode) {
+    if (!tc.use) return "k_chunk";
+    if (forward_cmma(tc, mode)) return "k_cmma";
+    switch (tc.family) {
+        case 1: return "k_small";
+        case 2: return tc.D == 32 && tc.variant >= 2 ? (mode == MODE_LOCAL ? "k_tiletc" : "k_mma32") : "k_tile";
+        case 3: return "k_bigtc";
+        case 4: return "k_col";
+        default: return "k_dense";
+    }
+}
+
+int kernel_ctas_per_sm(const TunedChoice& tc, int variant, int mode) {
+    if (!tc.use) return generic_ctas_per_sm(variant % GENERIC_VARIANTS);
+    if (forward_cmma(tc, mode)) return cmma_ctas_per_sm(tc.D);
+    return tc.family == 2 || tc.family == 3 ? tc.ctas_per_sm : 0;
+}
+
 cudaError_t prepare_tuned(const TunedChoice& tc, int rule, int mode) {
     if (!tc.use) return cudaSuccess;
     LaunchArgs none{};

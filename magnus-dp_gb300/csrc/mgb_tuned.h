@@ -56,7 +56,8 @@ int big_variants(int D);
 int big_ctas_per_sm(int D, int variant);
 // Group-tiled kernel (mgb_tuned.cu), variant 0: 2 CTAs per SM, 1: one;
 // at d = 32 variant 2: the tcgen05 forward local pass (mgb_tiletc.cu) with
-// the warp-MMA VJP, variant 3: the warp-MMA kernel for both.
+// the warp-MMA VJP (mgb_mma32.cu), variant 3: the warp-MMA forward pass
+// (mgb_cmma.cu, launch_cmma) with it.
 cudaError_t launch_tile(int D, int rule, int mode, const LaunchArgs& a, int grid, int variant, bool prepare_only);
 cudaError_t launch_tiletc(int rule, const LaunchArgs& a, int grid, bool prepare_only);
 // Warp-MMA VJP kernel at d = 32 (mgb_mma32.cu); two CTAs per SM.
@@ -75,6 +76,10 @@ cudaError_t launch_wait_selftest(uint64_t limit_ns, cudaStream_t st);
 // after them).
 constexpr int GENERIC_VARIANTS = 3;
 int generic_ctas_per_sm(int variant);
+// The kernel a choice runs for a pass, and the CTAs per SM its grid is bounded
+// to (0: as many as the chunks ask for).
+const char* kernel_name(const TunedChoice& tc, int mode);
+int kernel_ctas_per_sm(const TunedChoice& tc, int variant, int mode);
 // 1 if a kernel gave up a bounded device-side wait since the last call.
 int read_clear_device_timeout();
 cudaError_t prepare_tuned(const TunedChoice& tc, int rule, int mode);
