@@ -551,7 +551,8 @@ cudaError_t launch_big(int D, int rule, int mode, const LaunchArgs& a, int sms, 
     }
     switch (variant) {
         case 1: return launch_m<64, 64, 2>(rule, mode, a, grid, prepare_only);
-        case 2: return launch_r<64, 64, MODE_VJP, 2, 2>(rule, a, grid, prepare_only);
+        case 2:  // (the forward pass goes by launch_cmma)
+            return mode == MODE_VJP ? launch_r<64, 64, MODE_VJP, 2, 2>(rule, a, grid, prepare_only) : cudaErrorInvalidValue;
         case 3: return launch_m<64, 64, 1>(rule, mode, a, grid, prepare_only);
         case 4: return launch_m<64, 32, 3, 1>(rule, mode, a, grid, prepare_only);
         default: return launch_m<64, 32, 2>(rule, mode, a, grid, prepare_only);
