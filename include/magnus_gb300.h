@@ -64,8 +64,14 @@ enum { MGB_KIND_MATRIX = 0, MGB_KIND_SPACECURVE = 1 };
  * mgb_fwd_vjp_host_batched). */
 enum { MGB_DTYPE_F32 = 0, MGB_DTYPE_F64 = 1, MGB_DTYPE_C64 = 2, MGB_DTYPE_C128 = 3 };
 /* PLAIN: every product and sum in FP64 (parity form, <=1e-12 vs the reference).
- * MIXED: per-sample products and in-chunk prefixes in FP32, chunk carries,
- *        scans and the final Omega assembly in FP64. */
+ * MIXED: per-sample products and in-chunk prefixes in FP32 (compensated),
+ *        final Omega assembly in FP64.  Chunk carries and scans in FP64, or,
+ *        for SpaceCurve and d = 2 up to order 8 and for d = 16, 32, 64 and 128
+ *        (64, 128: up to order 6), in double-FP32: pairs of floats, about 48
+ *        significant bits, with FP32's exponent range.
+ * Results depend on the split of the samples over the GPU: the rounding of a
+ * trajectory may differ (within the forms' accuracy) between batches, and
+ * between GPUs, that make a call's chunks more or fewer. */
 enum { MGB_PRECISION_PLAIN = 0, MGB_PRECISION_MIXED = 1 };
 enum { MGB_OP_ONE = 0, MGB_OP_MANY = 1, MGB_OP_SUM = 2 };
 enum { MGB_INTEGRATOR_BOOLE = 0, MGB_INTEGRATOR_SIMPSON = 1, MGB_INTEGRATOR_TRAPEZOID = 2, MGB_INTEGRATOR_RIEMANN = 3 };
@@ -91,7 +97,11 @@ mgb_status mgb_forward(const mgb_problem* p, const void* A, void* out, void* car
 
 /* VJP: dA <- d<cot, op(Omega)>/dA (bilinear pairing, as the reference).
  * ckpt: buffer written by mgb_forward for the same problem and A, or NULL to
- * recompute the forward checkpoints. */
+ * recompute the forward checkpoints.  (Where checkpoint_K is 0, a call that
+ * keeps its checkpoints to itself may take a shorter interval than
+ * mgb_checkpoint_bytes counts with: d = 64 and 128 in the mixed form, multiples
+ * of 16 in the plain form, few chunks.  The two VJPs then agree to rounding, not
+ * bit for bit.) */
 mgb_status mgb_vjp(const mgb_problem* p, const void* A, const void* cot, const void* ckpt, void* dA, void* stream);
 
 /* Bytes of the checkpoint buffer for problem p (0 on invalid p). */

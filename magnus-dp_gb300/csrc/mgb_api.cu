@@ -144,18 +144,21 @@ int rule_divisibility(int integrator) {
     }
 }
 
-// Checkpoint interval.  The mixed form's chunk scans are FP64 (n(n-1)/2
-// products per chunk against (n-1)K FP32 products inside it), so it takes
-// long chunks at every d; the plain form keeps shorter ones at large d,
-// where its slots are twice as large and its scans cost little.
+// Checkpoint interval.  The mixed form's chunk scans (double-FP32 or FP64:
+// n(n-1)/2 products per chunk against (n-1)K FP32 products inside it) cost
+// several times a product of the chunk kernels, so it takes long chunks at
+// every d; the plain form keeps shorter ones at large d, where its slots are
+// twice as large and its scans cost little.
 int default_K(const mgb_problem& p) {
     // 4-element algebras (SpaceCurve, 2 x 2) in the mixed form with long
-    // sample runs: 1024.  Their FP32 chunk kernel (one thread per chunk) is
-    // cheap per sample, while every chunk step of the FP64 scan costs
-    // n(n-1)/2 products on the 1/64-rate FP64 pipe; four times fewer steps,
-    // and still 64+ chunks per instance for the thread-per-chunk parallelism.
-    // (The plain form's FP64 chunk kernel is the larger cost: it keeps 256
-    // and the parallelism.)
+    // sample runs: 1024.  Their FP32 chunk kernel is cheap per sample, while the
+    // scan walks an instance's chunks one after the other (one warp each); lanes
+    // make up for the fewer chunks.  At 256 and 1024, forward: 4096 curves of
+    // 65537 samples, n = 6, 2.81 and 2.34 ms; 64 of them 0.375 and 0.223; 16 2 x 2
+    // trajectories of 131073, n = 6, 0.473 and 0.210.  With the gradient 64 curves
+    // 1.19 and 0.94, 1024 of them 6.5 and 6.7; 1024 2 x 2 trajectories, n = 4, lose
+    // (forward 0.82 and 0.99, both 4.6 and 5.0).  (The plain form's FP64 chunk
+    // kernel is the larger cost: it keeps 256 and the parallelism.)
     if ((p.kind == MGB_KIND_SPACECURVE || p.dim == 2) && p.precision == MGB_PRECISION_MIXED && p.samples - 1 >= 65536)
         return 1024;
     if (p.kind == MGB_KIND_SPACECURVE || p.dim <= 32 || p.precision == MGB_PRECISION_MIXED) return 256;

@@ -1,6 +1,6 @@
 // Chunk kernel for d = 9..32 where no tensor-core kernel serves (the plain
-// form, float64 data, other dimensions), both precision forms: variant 0 of
-// the generic kernel at these dimensions.
+// form from d = 16, and in the mixed form float64 data and other dimensions):
+// one of the generic kernel's variants there (dense_variant in mgb_tuned.cu).
 //
 // One CTA per chunk, four samples at a time, all levels per group.  A thread
 // owns a 1 x 4 tile of the matrices at all four samples, so that W = A P
@@ -16,8 +16,9 @@
 // S = 8193, n = 4: 17.2 -> 8.1 / 53.7 -> 22.3 ms (one chunk per SM on 128 of
 // them: the pipe's own time is 7.6 ms forward); d = 16, 16 trajectories: 5.7 ->
 // 4.6 / 16.8 -> 12.3.  FP32, 64 trajectories of d = 24, n = 6: 25.6 -> 8.4 / 88.6
-// -> 43.5 ms.  Where half of a CTA's threads have no tile (d = 9, 12) the
-// level-major kernel is the faster one and the autotuner keeps it.
+// -> 43.5 ms.  Where half of a CTA's threads have no tile or there is one
+// warp of them (d = 9..12) the level-major kernel is the faster one for small calls,
+// and in FP64 for all below d = 16.
 #pragma once
 
 #include <algorithm>

@@ -567,7 +567,7 @@ cudaError_t launch_generic_chunk(bool fp64, int kind, int rule, int mode, const 
 
 template <class TS, int KIND, int G>
 static cudaError_t launch_small_g(int which, const InstDev* insts, int count, int f64io, int write_out, cudaStream_t st) {
-    // instances per CTA: as many as leave a CTA for each SM
+    // instances per CTA: as many as leave two CTAs for each SM
     int dev = 0, sms = 1;
     if (G < NT) {
         cudaError_t e = cudaGetDevice(&dev);

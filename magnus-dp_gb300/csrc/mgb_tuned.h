@@ -11,7 +11,7 @@ namespace mgb {
 
 struct TunedChoice {
     bool use = false;
-    int family = 0;  // 1: registers, one to 32 lanes per chunk (d = 2, SpaceCurve); 2: group-tiled CTA kernel (mixed, d = 16 / 32); 3: tensor-core level-major (mixed, d = 64 / 128); 4 / 5: one thread per column (d = 3..8) / per 1 x 4 tile (d = 9..32), variant 0 of the generic kernel
+    int family = 0;  // 1: registers, one to 32 lanes per chunk (d = 2, SpaceCurve); 2: group-tiled CTA kernel (mixed, d = 16 / 32); 3: tensor-core level-major (mixed, d = 64 / 128); 4 / 5: one thread per column (d = 3..8) / per 1 x 4 tile (d = 9..32), beside the generic kernel's variants
     int D = 0;
     int nmax = 0;
     int ctas_per_sm = 1;
@@ -35,8 +35,9 @@ int small_family_max_levels();
 // Column kernel for d = 3..8 (mgb_col.cuh): whether an order fits, teams per
 // chunk, VJP scratch (elements) wanted and needed.
 bool col_ok(bool plain, int D, int nmax);
-// Kernel for d = 9..32 outside the tensor-core kernels (mgb_dense.cuh); its
-// VJP runs in the generic kernel's slots.
+// Kernel for d = 9..32 outside the tensor-core kernels (mgb_dense.cuh; where it
+// stands among the variants: dense_variant in mgb_tuned.cu); its VJP runs in the
+// generic kernel's slots.
 bool dense_ok(bool plain, int d, int nmax);
 cudaError_t launch_dense(bool plain, int d, int rule, int mode, const LaunchArgs& a, int nmax, bool prepare_only);
 int col_lanes(bool plain, int D, int nmax, int64_t nwork, int64_t kmax, int sms);
@@ -49,8 +50,9 @@ int64_t small_family_slot(int64_t kmax, int lpc);
 TunedChoice choose_tuned(bool plain, int kind, int rule, int mode, bool f64io, const std::vector<InstDev>& hi,
                          int variant);
 // Tensor-core chunk kernel (mgb_bigtc.cu) for the mixed form at d = 64 / 128.
-// Variants: d = 64: k-block 32 or 64 x 2 or 1 CTAs per SM; d = 128: k-block
-// 32 or 64.  The grid is min(a.grid, sms x CTAs per SM).
+// Variants: d = 64: 0 and 1 k-block 32 or 64 at 2 CTAs per SM, 2 the VJP of 1 (its
+// forward pass is launch_cmma's), 3 k-block 64 at 1, 4 k-block 32 at 3; d = 128:
+// k-block 32 or 64, or 32 with 2 CTAs per SM.  The grid is min(a.grid, sms x CTAs per SM).
 cudaError_t launch_big(int D, int rule, int mode, const LaunchArgs& a, int sms, int variant, bool prepare_only);
 int big_variants(int D);
 int big_ctas_per_sm(int D, int variant);

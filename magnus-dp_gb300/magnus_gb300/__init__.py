@@ -17,7 +17,7 @@ Differences from the reference, by design:
   lanes are folded into the engine's algebra ("threadpool" is only valid
   inside a JAX FFI call, as in the reference).
 * Extra keyword ``precision``: ``"plain"`` (FP64 everywhere; the parity form)
-  or ``"mixed"`` (FP32 per-sample products, FP64 carries and sums).
+  or ``"mixed"`` (FP32 per-sample products, carries in FP64 or pairs of floats).
 * ``compute_vjp(vjp_data=...)`` checks the carry's shape exactly like the
   reference and then recomputes what it needs from the chunk checkpoints
   (replaying the forward costs less than reading Q*(n-1)*S*d*d values).

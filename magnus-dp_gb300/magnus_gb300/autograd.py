@@ -33,7 +33,9 @@ def _chunk_interval(kind, prec, dim, Ab):
     fewer chunks than SMs, they are halved: d = 64 and 128 in the mixed form,
     down to 64 (one d = 128 trajectory of 4097 samples, n = 4, forward and
     backward: 41.4 -> 14.2 ms), and multiples of 16 in the plain form, down to
-    32, while they still fit one to an SM."""
+    32, while they still fit one to an SM.  (The checkpoints that wait for the
+    backward pass grow with the chunks: up to four times in the mixed form and
+    eight in the plain one, on calls of few chunks: 17 -> 68 MB for that trajectory.)"""
     mixed = prec == _lib.PRECISION_MIXED
     if kind != _lib.KIND_MATRIX or Ab.shape[1] < 2 or not (dim in (64, 128) if mixed else dim >= 16 and dim % 16 == 0):
         return 0
