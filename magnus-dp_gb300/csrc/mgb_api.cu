@@ -777,7 +777,7 @@ LaunchArgs seg_args(const PlanCore& pc, const Segment& sg, cudaStream_t st) {
 // that what a call of a few chunks measured does not decide for a full one
 // (d = 16 FP64, 32 trajectories after a single one: 11.2 ms on the level-major
 // kernel that suited the single one, 8.5 on the tile kernel).  MGB_AUTOTUNE=0
-// turns tuning off (variant 0 everywhere); MGB_FORCE_VARIANT=k forces variant
+// turns tuning off (untimed_variant: variant 0 but for d = 3..8); MGB_FORCE_VARIANT=k forces variant
 // k (tests use it to check every variant against the oracle).
 struct TuneKey {
     int mode, family, D, rule, nmax, plain, kind, f64io, lpc, load, len;
@@ -914,6 +914,8 @@ mgb_status plan_autotune(PlanCore& pc, cudaStream_t st) {
             sg.variant = sg.vjp_variant = forced < nv ? forced : 0;
             continue;
         }
+        sg.variant = untimed_variant(tc0, pc.plain, MODE_LOCAL, sg.nmax, sg.nwork, pc.sms);
+        sg.vjp_variant = untimed_variant(tc0, pc.plain, MODE_VJP, sg.nmax, sg.nwork, pc.sms);
         if (nv <= 1 || !enabled) continue;
         const int load = sg.nwork < pc.sms ? 0 : sg.nwork <= 8LL * pc.sms ? 1 : 2;
         int len = 0;
@@ -949,9 +951,9 @@ mgb_status plan_autotune(PlanCore& pc, cudaStream_t st) {
             return MGB_OK;
         };
         mgb_status s = pick(MODE_LOCAL, sg.variant, sg.tune_ms);
-        sg.vjp_variant = sg.variant;
         const bool kernels = tc0.use ? tc0.family >= 4 : nv > GENERIC_VARIANTS;  // the variants are different kernels
-        if (s == MGB_OK && pc.has_vjp && kernels) s = pick(MODE_VJP, sg.vjp_variant, sg.vjp_ms);
+        if (!kernels) sg.vjp_variant = sg.variant;
+        else if (s == MGB_OK && pc.has_vjp) s = pick(MODE_VJP, sg.vjp_variant, sg.vjp_ms);
         if (s != MGB_OK) return s;
     }
     return MGB_OK;
@@ -2029,7 +2031,8 @@ extern "C" mgb_status mgb_forward_noalloc(const mgb_problem* p, const void* A, v
     la.kmax = L - 1;
     la.f64io = f64io;
     la.stream = cs;
-    MGB_CUDA_TRY(launch_chunk_any(plain, p->kind, p->integrator, MODE_LOCAL, la, hi, di.sms, 0));
+    MGB_CUDA_TRY(launch_chunk_any(plain, p->kind, p->integrator, MODE_LOCAL, la, hi, di.sms,
+                                  untimed_variant(tc, plain, MODE_LOCAL, (int)p->n, v.C, di.sms)));
     MGB_CUDA_TRY(launch_small(true, p->kind, SMALL_SCAN, d_inst, 1, f64io, 0, (int64_t)p->n * v.m, cs));
     MGB_CUDA_TRY(launch_small(true, p->kind, SMALL_FIN_FWD, d_inst, 1, f64io, 1, (int64_t)p->n * v.m, cs));
     return MGB_OK;

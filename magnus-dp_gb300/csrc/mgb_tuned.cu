@@ -599,6 +599,23 @@ TunedChoice choose_tuned(bool plain, int kind, int rule, int mode, bool f64io, c
     return tc;
 }
 
+// Column kernel (d = 3..8) or level-major kernel untimed, for calls of fewer
+// chunks than SMs: the composition of a chunk's runs grows with n^2, and the
+// VJP pays it both ways.  One trajectory of S = 16385, level-major time over the
+// column kernel's: forward n = 6 0.99 (d = 6 FP64) to 2.0, n = 8 0.85..1.2 from d = 5
+// on (d = 3, 4: 1.2..1.8), n = 12 0.74..1.0; VJP in FP32 n = 5 1.0..1.4 and n = 6
+// 0.92..1.0, but 0.79 and 0.83 from n = 4 on at d = 5 and 6, and 1.26 still at d = 8;
+// in FP64 n = 8 1.27 at d = 3, n = 6 1.1 at d = 4, 0.9 at d = 5..7 and 0.69 at d = 8,
+// where n = 5 is 0.90.
+int untimed_variant(const TunedChoice& tc0, bool plain, int mode, int nmax, int64_t nwork, int sms) {
+    if (!tc0.use || tc0.family != 4 || nwork >= sms) return 0;
+    const int d = tc0.D, all = nmax;
+    // the highest order of the column kernel's
+    const int fp64[6] = {all, 6, 5, 5, 5, 4}, fp32[6] = {8, 5, 3, 3, 5, 8};
+    const int most = mode == MODE_LOCAL ? (d <= 4 ? all : 6) : (plain ? fp64 : fp32)[d - 3];
+    return nmax <= most ? 0 : 1;
+}
+
 // d = 32 variant 3 and d = 64 variant 2 run their forward local pass on k_cmma
 static bool forward_cmma(const TunedChoice& tc, int mode) {
     return mode == MODE_LOCAL && ((tc.family == 2 && tc.D == 32 && tc.variant == 3) || (tc.family == 3 && tc.D == 64 && tc.variant == 2));

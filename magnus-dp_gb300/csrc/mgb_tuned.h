@@ -78,6 +78,8 @@ cudaError_t launch_wait_selftest(uint64_t limit_ns, cudaStream_t st);
 // after them).
 constexpr int GENERIC_VARIANTS = 3;
 int generic_ctas_per_sm(int variant);
+// The variant a pass runs where nothing is timed (tc0: variant 0's choice).
+int untimed_variant(const TunedChoice& tc0, bool plain, int mode, int nmax, int64_t nwork, int sms);
 // The kernel a choice runs for a pass, and the CTAs per SM its grid is bounded
 // to (0: as many as the chunks ask for).
 const char* kernel_name(const TunedChoice& tc, int mode);

@@ -1,5 +1,5 @@
-"""Variant 0 of a chunk kernel runs where nothing is timed (MGB_AUTOTUNE=0, the
-allocation-free forward, inside a capture): it is not the slow one."""
+"""The chunk-kernel variant that runs where nothing is timed (MGB_AUTOTUNE=0, the
+allocation-free forward, inside a capture) is not the slow one."""
 import ctypes
 
 import pytest
@@ -9,12 +9,14 @@ from magnus_gb300 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("precision,dims", [("plain", (9, 10, 12, 15)), ("mixed", (9, 10, 12))])
-def test_untimed_variant_is_not_slow(precision, dims, cuda, monkeypatch):
-    """One trajectory, the best of five passes: variant 0 within a quarter of the
-    fastest variant, forward and backward."""
+@pytest.mark.parametrize("precision,n,dims", [("plain", 3, (9, 10, 12, 15)), ("mixed", 3, (9, 10, 12)),
+                                              ("plain", 8, (3, 6, 8)), ("mixed", 12, (3, 6, 7)), ("mixed", 4, (5, 6, 8))])
+def test_untimed_variant_is_not_slow(precision, n, dims, cuda, monkeypatch):
+    """One trajectory, the best of five passes: the untimed choice within a quarter of
+    the fastest variant, forward and backward."""
     import torch
-    lib, S, n = _lib.load(), 4097, 3
+    monkeypatch.setenv("MGB_AUTOTUNE", "0")
+    lib, S = _lib.load(), 4097
     f64 = precision == "plain"
     for d in dims:
         torch.manual_seed(d)
@@ -25,8 +27,10 @@ def test_untimed_variant_is_not_slow(precision, dims, cuda, monkeypatch):
                                  dim=d, t0=0.0, tf=1.0)
         one = lambda t: (ctypes.c_void_p * 1)(t.data_ptr())  # noqa: E731
         times = []
-        for v in range(4):
-            monkeypatch.setenv("MGB_FORCE_VARIANT", str(v))
+        for v in (None, 0, 1, 2, 3):
+            monkeypatch.delenv("MGB_FORCE_VARIANT", raising=False)
+            if v is not None:
+                monkeypatch.setenv("MGB_FORCE_VARIANT", str(v))
             plan = ctypes.c_void_p()
             _lib.check(lib.mgb_plan_create(ctypes.byref(prob), 1, one(A), one(out), one(cot), one(dA), ctypes.byref(plan)))
             best = [1e9, 1e9]
